@@ -640,7 +640,7 @@ __device__ __forceinline__ void stage_run(const StageArgs& a) {
           };
           auto pair = [&](const R (&x)[5], const R (&y)[5]) {
             return weno5x2(make_float2(x[0], y[0]), make_float2(x[1], y[1]), make_float2(x[2], y[2]),
-                           make_float2(x[3], y[3]), make_float2(x[4], y[4]), K.textbook);
+                           make_float2(x[3], y[3]), make_float2(x[4], y[4]), 0);
           };
           auto first4 = [&](const R (&u)[5][5], R (&wm)[5]) {
             const float2 r01 = pair(u[0], u[1]), r23 = pair(u[2], u[3]);
@@ -657,8 +657,6 @@ __device__ __forceinline__ void stage_run(const StageArgs& a) {
               return;
             }
             Prim5<R> pm = cons2prim<R, EX>(wm[0], wm[1], wm[2], wm[3], wm[4], K.gm1);
-            if (K.textbook && !admissible(pm))
-              pm = cons2prim<R, EX>(u[0][2], u[1][2], u[2][2], u[3][2], u[4][2], K.gm1);
             sN[0 * NN + w] = pm.r;
             sN[1 * NN + w] = pm.u;
             sN[2 * NN + w] = pm.v;
@@ -724,10 +722,6 @@ __device__ __forceinline__ void stage_run(const StageArgs& a) {
             } else {
               zWm_cur = cons2prim<R, EX>(wz[0], wz[1], wz[2], wz[3], wz[4], K.gm1);
               zWcur = zWm_cur;
-              if (K.textbook && !admissible(zWm_cur)) {
-                zWm_cur = cons2prim<R, EX>(zw[2][0], zw[2][1], zw[2][2], zw[2][3], zw[2][4], K.gm1);
-                zWcur = zWm_cur;
-              }
             }
           }
           if (do_xy) __syncthreads();
@@ -739,7 +733,7 @@ __device__ __forceinline__ void stage_run(const StageArgs& a) {
           for (int v = 0; v < 5; ++v)
 #pragma unroll
             for (int s = 0; s < 5; ++s) u[v][s] = zw[s][v];
-          weno5_node<R, EX, TB>(u, K.textbook, wm, wp);
+          weno5_node<R, EX, TB>(u, TB ? 1 : 0, wm, wp);
           if constexpr (C::SP) {
             R ir;
             const Prim5<R> pz = cons2prim_ir<R>(wm[0], wm[1], wm[2], wm[3], wm[4], K.gm1, ir);
@@ -751,7 +745,7 @@ __device__ __forceinline__ void stage_run(const StageArgs& a) {
             zWcur = cons2prim<R, EX>(wp[0], wp[1], wp[2], wp[3], wp[4], K.gm1);
           else
             zWcur = zWm_cur;
-          if (K.textbook && !(admissible(zWm_cur) && admissible(zWcur))) {
+          if (TB && !(admissible(zWm_cur) && admissible(zWcur))) {
             const Prim5<R> pc = cons2prim<R, EX>(zw[2][0], zw[2][1], zw[2][2], zw[2][3], zw[2][4], K.gm1);
             if (!admissible(zWm_cur)) zWm_cur = pc;
             if (!admissible(zWcur)) zWcur = pc;
@@ -807,7 +801,7 @@ __device__ __forceinline__ void stage_run(const StageArgs& a) {
                 for (int s = 0; s < 5; ++s) u[v][s] = pl[v * PLS + base + s * PWS];
             }
             R wm[5], wp[5];
-            weno5_node<R, EX, TB>(u, K.textbook, wm, wp);
+            weno5_node<R, EX, TB>(u, TB ? 1 : 0, wm, wp);
             if constexpr (C::SP) {
               R ir;
               const Prim5<R> pm = cons2prim_ir<R>(wm[0], wm[1], wm[2], wm[3], wm[4], K.gm1, ir);
@@ -815,7 +809,7 @@ __device__ __forceinline__ void stage_run(const StageArgs& a) {
               continue;
             }
             Prim5<R> pm = cons2prim<R, EX>(wm[0], wm[1], wm[2], wm[3], wm[4], K.gm1);
-            if (K.textbook && !admissible(pm))
+            if (TB && !admissible(pm))
               pm = cons2prim<R, EX>(u[0][2], u[1][2], u[2][2], u[3][2], u[4][2], K.gm1);
             constexpr int NN = C::NXN + C::NYN;
             sN[0 * NN + w] = pm.r;
