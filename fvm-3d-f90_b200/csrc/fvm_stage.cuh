@@ -847,12 +847,28 @@ __device__ __forceinline__ void stage_run(const StageArgs& a) {
         // pair per cell (scheme_reconstruct_MUSCL.f90:114-226); TEXTBOOK
         // falls back to the cell value where a state is not admissible
         auto node = [&](const R (&p)[5][3], R (&qr)[5], R (&ql)[5]) {
+          if constexpr (sizeof(R) == 8 && !EX) {
+            auto lim = [&](auto L) {
 #pragma unroll
-          for (int v = 0; v < 5; ++v) {
-            R Dbm, Dbp;
-            muscl_slopes<R, EX>(p[v][0], p[v][1], p[v][2], K.limiter, Dbm, Dbp);
-            qr[v] = p[v][1] + R(0.25) * (K.omk * Dbm + K.opk * Dbp);
-            ql[v] = p[v][1] - R(0.25) * (K.omk * Dbp + K.opk * Dbm);
+              for (int v = 0; v < 5; ++v)
+                muscl_node_fp64<decltype(L)::value>(p[v][0], p[v][1], p[v][2], K.omk, K.opk, qr[v], ql[v]);
+            };
+            if (K.limiter == LIM_MINMOD_)
+              lim(std::integral_constant<int, LIM_MINMOD_>());
+            else if (K.limiter == LIM_VANLEER_)
+              lim(std::integral_constant<int, LIM_VANLEER_>());
+            else if (K.limiter == LIM_VANALBADA_)
+              lim(std::integral_constant<int, LIM_VANALBADA_>());
+            else
+              lim(std::integral_constant<int, LIM_NONE_>());
+          } else {
+#pragma unroll
+            for (int v = 0; v < 5; ++v) {
+              R Dbm, Dbp;
+              muscl_slopes<R, EX>(p[v][0], p[v][1], p[v][2], K.limiter, Dbm, Dbp);
+              qr[v] = p[v][1] + R(0.25) * (K.omk * Dbm + K.opk * Dbp);
+              ql[v] = p[v][1] - R(0.25) * (K.omk * Dbp + K.opk * Dbm);
+            }
           }
           if (K.textbook) {
             if (!admissible(mkprim(qr)))
