@@ -52,6 +52,64 @@ inline void equal_chunks(int64_t nz, int64_t L, std::vector<int64_t>& z0s) {
   z0s.push_back(nz);
 }
 
+// A z column of one tile.
+struct ZColumn {
+  int blk, x0, y0, nz;
+};
+
+// Cut the columns into equal chunks of at most L planes.
+void chunk_columns(const std::vector<ZColumn>& cols, int64_t L, std::vector<Task>& out) {
+  std::vector<int64_t> z0s;
+  for (const auto& c : cols) {
+    equal_chunks(c.nz, L, z0s);
+    for (size_t i = 0; i + 1 < z0s.size(); ++i) out.push_back({c.blk, c.x0, c.y0, (int)z0s[i], (int)z0s[i + 1], 0});
+  }
+}
+
+// Even split of z columns over `slots` resident CTAs: the columns, taken one
+// after the other, are cut wherever a CTA's share of the work is full, so all
+// shares are the same to within a plane or two and a stage is one round of the
+// queue (equal chunks leave CTAs idle in its last round: 2.3 rounds on the
+// 128^3 vortex, 0.8 of one on a 61x83x47 blast). A piece of c planes costs
+// c + ovh plane-times (the z window's warm-up and the set-up) and has at least
+// kMinPiece planes where the column allows it. The smallest share that fits is
+// found by growing it from the mean: O(pieces) per try, a few tries, so the
+// re-plans of a serving loop stay cheap. Measured per step, equal chunks of
+// the length a queue estimate picked -> even split: vortex 128^3 FP64 926 ->
+// 909 us, 64^3 172 -> 153; Taylor-Green 128^3 FP64 877 -> 833, 30^3 FP32 96 ->
+// 74; 61x83x47 blast FP64 159 -> 138; 24 mixed FP32 cases 1143 -> 1086. The
+// pieces' least length (1 to 3) and ovh (0.6 to 1.4 for WENO) move these by
+// less than 2 %. Returns the share.
+double even_split(const std::vector<ZColumn>& cols, int slots, double ovh, std::vector<Task>& out) {
+  constexpr int kMinPiece = 2, kTries = 400;
+  double total = 0.0;
+  for (const auto& c : cols) total += c.nz;
+  const size_t first = out.size();
+  double share = std::max(total / slots, (double)kMinPiece) + ovh;
+  for (int it = 0; it < kTries; ++it, share += std::max(0.25, share / 128.0)) {
+    out.resize(first);
+    int used = 1;
+    double left = share;
+    for (const auto& c : cols) {
+      for (int z = 0; z < c.nz;) {
+        if (left < ovh + std::min(kMinPiece, c.nz - z)) {
+          ++used;
+          left = share;
+        }
+        int n = std::min(c.nz - z, std::max(kMinPiece, (int)(left - ovh)));
+        const int rest = c.nz - z - n;
+        if (rest > 0 && rest < kMinPiece) n += n >= 2 * kMinPiece - rest ? rest - kMinPiece : rest;
+        out.push_back({c.blk, c.x0, c.y0, z, z + n, 0});
+        z += n;
+        left -= n + ovh;
+      }
+      if (used > slots && it + 1 < kTries) break;  // does not fit: a larger share
+    }
+    if (used <= slots) break;
+  }
+  return share;
+}
+
 // Makespan of the persistent work queue for tasks of the given costs on
 // `slots` CTAs: tasks are taken longest first, each by the CTA that frees
 // first (what the atomic task counter does when costs are uniform per plane).
@@ -714,8 +772,22 @@ int Engine::plan() {
       // blocks are at least 32 wide, else 16 x 16 (exact) / 16 x 8
       int64_t minx = 1 << 30;
       for (int b : hc.blocks) minx = std::min(minx, blocks[b].n[0]);
+      // the reference's WENO5 + AUSM in FP32: its side values make the wider
+      // tile's smaller halo pay (vortex 128^3: 634 against 674 us per step, 64^3
+      // 120 against 126, 160^3 1107 against 1222) while its padding does not
+      // cost more than the 6 % it gains
+      int64_t pad2 = 0, pad3 = 0;
+      for (int b : hc.blocks) {
+        const int64_t* n = blocks[b].n;
+        pad2 += round_up(n[0], 32) * round_up(n[1], 8) * n[2];
+        pad3 += round_up(n[0], 16) * round_up(n[1], 8) * n[2];
+      }
+      const bool wide32 = prec == FVM_PREC_FP32_FLUX && dim == 3 && c.reconstruct == FVM_RECON_WENO && !tb &&
+                          c.flux_split == FVM_FLUX_AUSM && 0.94 * (double)pad2 <= (double)pad3;
       if (prec == FVM_PREC_FP64_EXACT)
         tile = minx >= 32 ? 2 : 1;
+      else if (wide32)
+        tile = 2;
       else
         tile = (dim == 2 && minx >= 32) ? 2 : 3;
     }
@@ -759,70 +831,35 @@ int Engine::plan() {
     Group& G = groups[g];
     G.task_off = (int)tasks.size();
     std::vector<Task> gt;
-    // z chunk of the group's cases without a tuned one: the length with the
-    // lowest estimated queue makespan over all the group's tasks. A task of c
-    // planes costs c plane-times plus the warm-up of its z window (WENO: 2
-    // planes of z-only work, MUSCL 1) and its set-up; the queue of T tasks of
-    // total cost S and longest cost M on the kernel's resident CTAs takes M
-    // while T fits on them, else about S / CTAs + (M / 2) (CTAs / T): taken
-    // longest first, the queue ends on short tasks, the more so the more
-    // tasks each CTA takes (on the 64-case batch the estimate picks the
-    // longest chunks, as measured best). Alone, a small case takes short
-    // chunks to spread over the CTAs; in a large batch the warm-ups dominate
-    // and the chunks grow. The estimate costs O(blocks) per candidate, so
-    // the re-plans of a serving loop stay cheap. The state does not depend
-    // on the tiling (only the residual norms' summation order does).
-    int64_t L_auto = 0;
-    if (G.dim == 3) {
-      auto in_group = [&](int ci) { return cases[ci].group == (int)g; };
-      const double ovh = G.recon == FVM_RECON_WENO ? 1.0 : (G.recon == FVM_RECON_MUSCL ? 0.65 : 0.35);
-      struct QStat {
-        double tasks = 0, sum = 0, mx = 0;
-      };
-      auto add_case = [&](const HCase& hc, int64_t L, QStat& q) {
-        for (int bi : hc.blocks) {
+    // The cases without a tuned z chunk share the resident CTAs evenly
+    // (even_split); a task's warm-up and set-up cost about this many planes.
+    // The state does not depend on the tiling (only the residual norms'
+    // summation order does). In 2D a plane is a task of its own unless the
+    // planes outnumber the CTAs (a 21^2 case of two planes: 81 -> 47 us per
+    // step).
+    const double ovh = G.recon == FVM_RECON_WENO ? 1.0 : (G.recon == FVM_RECON_MUSCL ? 0.65 : 0.35);
+    std::vector<ZColumn> cols;
+    int64_t planes2d = 0;
+    for (int ci : live_cases)
+      if (cases[ci].group == (int)g && G.dim == 2)
+        for (int bi : cases[ci].blocks) {
           const HBlock& b = blocks[bi];
-          const int64_t ncol = ((b.n[0] + G.k.tx - 1) / G.k.tx) * ((b.n[1] + G.k.ty - 1) / G.k.ty);
-          const int64_t nc = std::max<int64_t>(1, (b.n[2] + L - 1) / L);  // equal_chunks
-          const int64_t longest = b.n[2] / nc + (b.n[2] % nc ? 1 : 0);
-          q.tasks += (double)(ncol * nc);
-          q.sum += (double)ncol * ((double)b.n[2] + (double)nc * ovh);
-          q.mx = std::max(q.mx, (double)longest + ovh);
+          planes2d += ((b.n[0] + G.k.tx - 1) / G.k.tx) * ((b.n[1] + G.k.ty - 1) / G.k.ty) * b.n[2];
         }
-      };
-      bool any_auto = false;
-      QStat fixed;
-      for (int ci : live_cases) {
-        if (!in_group(ci)) continue;
-        if (cases[ci].zchunk > 0)
-          add_case(cases[ci], cases[ci].zchunk, fixed);
-        else
-          any_auto = true;
-      }
-      double best = 0.0;
-      for (int64_t cand = 64; any_auto && cand >= 4; cand -= (cand > 16 ? 4 : 2)) {
-        QStat q = fixed;
-        for (int ci : live_cases)
-          if (in_group(ci) && cases[ci].zchunk <= 0) add_case(cases[ci], cand, q);
-        const double m = q.tasks <= G.grid ? q.mx : q.sum / G.grid + 0.5 * q.mx * G.grid / q.tasks;
-        if (L_auto <= 0 || m < best * 0.995) {
-          best = m;
-          L_auto = cand;
-        }
-      }
-    }
     for (int ci : live_cases) {
       HCase& hc = cases[ci];
       if (hc.group != (int)g) continue;
-      const int64_t L = hc.zchunk > 0 ? (int64_t)hc.zchunk : L_auto;
+      const bool even = G.dim == 3 && hc.zchunk <= 0;
       std::vector<int64_t> z0s;
       std::vector<Task> ct;
       for (int bi : hc.blocks) {
         const HBlock& b = blocks[bi];
-        if (G.dim == 3)
-          equal_chunks(b.n[2], L, z0s);
-        else
-          z0s = {0, b.n[2]};
+        if (even) {
+          for (int64_t y0 = 0; y0 < b.n[1]; y0 += G.k.ty)
+            for (int64_t x0 = 0; x0 < b.n[0]; x0 += G.k.tx) cols.push_back({bi, (int)x0, (int)y0, (int)b.n[2]});
+          continue;
+        }
+        equal_chunks(b.n[2], G.dim == 3 ? hc.zchunk : (planes2d + G.grid - 1) / G.grid, z0s);
         for (size_t c = 0; c + 1 < z0s.size(); ++c)
           for (int64_t y0 = 0; y0 < b.n[1]; y0 += G.k.ty)
             for (int64_t x0 = 0; x0 < b.n[0]; x0 += G.k.tx) {
@@ -842,7 +879,7 @@ int Engine::plan() {
       // more CTAs for a shorter time (each piece warms up its own z window).
       // It depends on the case and the kernel's slot count only, so a case
       // is tiled alike alone and batched.
-      if (G.dim == 3 && hc.tail_split > 1 && (int64_t)ct.size() > G.grid) {
+      if (G.dim == 3 && hc.zchunk > 0 && hc.tail_split > 1 && (int64_t)ct.size() > G.grid) {
         std::stable_sort(ct.begin(), ct.end(),
                          [](const Task& a, const Task& b) { return (a.z1 - a.z0) > (b.z1 - b.z0); });
         const size_t r = ct.size() % (size_t)G.grid;
@@ -864,6 +901,28 @@ int Engine::plan() {
         ct.insert(ct.end(), pieces.begin(), pieces.end());
       }
       gt.insert(gt.end(), ct.begin(), ct.end());
+    }
+    if (!cols.empty()) {
+      const size_t first = gt.size();
+      const double share = even_split(cols, G.grid, ovh, gt);
+      // The FP32 form reads its tile halos at a third of the HBM rate, so it
+      // gains from neighbouring columns marching in step (their halos meet in
+      // L2): equal chunks that fit one round and come within 8 % of the even
+      // share replace it (Taylor-Green 110^3 608 -> 592 us, 90^3 vortex 338 ->
+      // 332). The FP64 forms do not notice (112^3 blast 374 even, 412 chunked).
+      if (G.prec == FVM_PREC_FP32_FLUX) {
+        int64_t nz = 0;
+        for (const auto& c : cols) nz = std::max<int64_t>(nz, c.nz);
+        int64_t L = std::max<int64_t>(4, (int64_t)share - 1);
+        for (; L <= nz && (double)L + ovh <= 1.08 * share; ++L) {
+          int64_t n = 0;
+          for (const auto& c : cols) n += (c.nz + L - 1) / L;
+          if (n > G.grid) continue;
+          gt.resize(first);
+          chunk_columns(cols, L, gt);
+          break;
+        }
+      }
     }
     std::stable_sort(gt.begin(), gt.end(), [](const Task& a, const Task& b) { return (a.z1 - a.z0) > (b.z1 - b.z0); });
     tasks.insert(tasks.end(), gt.begin(), gt.end());

@@ -247,7 +247,9 @@ int fvm_case_state(fvm_ctx* ctx, int case_id, double* t, double* dt, int64_t* st
  * fvm_tune_set_tail_split (3D; split 1..8, 1 = off, the default): when the
  * case's tasks fill the stage kernel's resident CTAs k times and r more, its
  * r shortest tasks are cut along z into `split` pieces (of at least 2
- * planes), so the last, partial round of the work queue is shorter. */
+ * planes), so the last, partial round of the work queue is shorter; with the
+ * heuristic's z chunk the tasks already share the CTAs evenly and nothing is
+ * cut. */
 int fvm_tune_set(fvm_ctx* ctx, int case_id, int tile, int zchunk);
 int fvm_tune_set_tail_split(fvm_ctx* ctx, int case_id, int split);
 int fvm_tune_time_step(fvm_ctx* ctx, int reps, float* ms_per_step);
