@@ -80,7 +80,7 @@ constexpr int kPartStride = 8;
 struct StageArgs {
   const Task* tasks;
   int32_t ntasks;
-  int32_t* counter;            // work-queue head, zeroed before each launch
+  int32_t* counter;            // tasks taken from the queue beyond each CTA's first, zeroed before each launch
   const DevBlock* blocks;
   const DevCase* cases;
   const DevCaseState* cstate;
@@ -103,9 +103,10 @@ struct StageArgs {
 // kernel launched without the attribute). As every kernel of the chain waits,
 // the completion of one implies that of all before it. pdl_trigger() lets the
 // next launch be scheduled once every CTA of this one has started; it orders
-// no memory. Only the short gather and finalize kernels trigger early: a
-// launch scheduled behind a long kernel's tail places its CTAs on the few SMs
-// free at that moment (up to 8 gather CTAs per SM) and runs unbalanced.
+// no memory. Only the short gather and finalize kernels and one-round 2D stage
+// launches trigger early, after their own wait: a launch scheduled behind a
+// long kernel's tail places its CTAs on the few SMs free at that moment (up to
+// 8 gather CTAs per SM) and runs unbalanced.
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
