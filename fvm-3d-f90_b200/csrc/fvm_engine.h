@@ -178,6 +178,11 @@ class Engine {
   DevBlock* d_blocks_ = nullptr;
   DevCase* d_cases_ = nullptr;
   int* d_case_blk_ = nullptr;
+  // one allocation: kernel error flag (a tensor copy that did not arrive),
+  // padded to kStateHead, then the case states; h_state_ is its pinned copy
+  static constexpr size_t kStateHead = 64;
+  int fetch_states(int first, int last);
+  char* h_state_ = nullptr;
   DevCaseState* d_state_ = nullptr;
   int state_cap_ = 0;
   Task* d_tasks_ = nullptr;
@@ -190,7 +195,7 @@ class Engine {
   int vlist_off_[6] = {0, 0, 0, 0, 0, 0}, vlist_n_[6] = {0, 0, 0, 0, 0, 0};
   std::vector<CUtensorMap*> d_tmap_;  // per group: [block][role A..ACC][plane, z] (null: no TMA)
   std::vector<size_t> cap_tmap_;      // their capacities in maps (grown, never shrunk)
-  int32_t* d_err_ = nullptr;          // kernel error flag (a tensor copy that did not arrive)
+  int32_t* d_err_ = nullptr;          // head of the state allocation
   int* d_dtmask_ = nullptr;           // cases whose dt prepare() recomputes
   int dtmask_cap_ = 0;
   bool drop_copies_ = false;          // test hook: tensor copies armed but not issued
