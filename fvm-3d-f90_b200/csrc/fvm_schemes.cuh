@@ -205,14 +205,15 @@ __device__ __forceinline__ double rcp_twice_(double x) {
   const double r2 = __hiloint2double(__double2hiint(r) + (1 << 20), __double2loint(r));
   return fma(r2, fma(e, e, e), r2);
 }
+__device__ __forceinline__ double weno5_h(double D) { return fma(0.609375 * D, D, 0.75e-6); }
 template <bool TB>
-__device__ __forceinline__ WenoParts weno5_parts(double u0, double u1, double u2, double u3, double u4) {
+__device__ __forceinline__ WenoParts weno5_parts(double D01, double D12, double D23, double D34, double h12, double h23,
+                                                 double b1) {
   WenoParts w;
-  w.D01 = u1 - u0;
-  w.D12 = u2 - u1;
-  w.D23 = u3 - u2;
-  w.D34 = u4 - u3;
-  const double h12 = fma(0.609375 * w.D12, w.D12, 0.75e-6), h23 = fma(0.609375 * w.D23, w.D23, 0.75e-6);
+  w.D01 = D01;
+  w.D12 = D12;
+  w.D23 = D23;
+  w.D34 = D34;
   const double r0 = fma(-1.375, w.D12, w.D01), r2 = fma(-1.375, w.D23, w.D34);
   const double e0 = fma(r0, r0, h12), e2 = fma(r2, r2, h23);
   double e1;
@@ -220,7 +221,7 @@ __device__ __forceinline__ WenoParts weno5_parts(double u0, double u1, double u2
     const double r1 = fma(-0.625, w.D23, w.D12);
     e1 = fma(r1, r1, h23);
   } else {
-    const double a1 = w.D23 - w.D12, b1 = u1 + u3;
+    const double a1 = w.D23 - w.D12;
     e1 = fma((13.0 / 3.0) * a1, a1, fma(b1, b1, 4.0e-6));
   }
   const double d0 = e0 * e0, d1 = e1 * e1, d2 = e2 * e2;
@@ -229,11 +230,25 @@ __device__ __forceinline__ WenoParts weno5_parts(double u0, double u1, double u2
   w.P2 = d0 * d1;
   return w;
 }
+template <bool TB>
+__device__ __forceinline__ WenoParts weno5_parts(double u0, double u1, double u2, double u3, double u4) {
+  return weno5_parts<TB>(u1 - u0, u2 - u1, u3 - u2, u4 - u3, weno5_h(u2 - u1), weno5_h(u3 - u2), u1 + u3);
+}
 __device__ __forceinline__ double weno5_left(const WenoParts& w, double u2) {
   const double s0 = fma(5.0 / 12.0, w.D12, (-1.0 / 6.0) * w.D01);
   const double s1 = fma(0.5, w.D12, w.D23), s2 = fma(-0.25, w.D34, w.D23);
   const double num = fma(w.P0, s0, fma(w.P1, s1, w.P2 * s2));
   return fma(num, rcp_twice_(fma(3.0, w.P2, fma(6.0, w.P1, w.P0))), u2);
+}
+// Two neighbouring left-biased evaluations (u0..u4 and u1..u5, the reference's
+// form): three differences and one square are shared and six values are loaded
+// instead of ten.
+__device__ __forceinline__ void weno5_pair(double u0, double u1, double u2, double u3, double u4, double u5, double& a,
+                                           double& b) {
+  const double D12 = u2 - u1, D23 = u3 - u2, D34 = u4 - u3;
+  const double h23 = weno5_h(D23);
+  a = weno5_left(weno5_parts<false>(u1 - u0, D12, D23, D34, weno5_h(D12), h23, u1 + u3), u2);
+  b = weno5_left(weno5_parts<false>(D12, D23, D34, u5 - u4, h23, weno5_h(D34), u2 + u4), u3);
 }
 __device__ __forceinline__ double weno5_right(const WenoParts& w, double u2) {
   const double s0 = fma(5.0 / 12.0, w.D23, (-1.0 / 6.0) * w.D34);
@@ -304,6 +319,42 @@ __device__ __forceinline__ float2 weno5x2(float2 u0, float2 u1, float2 u2, float
   const float2 num = __ffma2_rn(P0, s0, __ffma2_rn(P1, S1, __fmul2_rn(P2, S2)));
   const float2 den = __ffma2_rn(f2_(6.0f), __fadd2_rn(P1, P2), P0);
   return __ffma2_rn(num, make_float2(rcp_(den.x), rcp_(den.y)), u2);
+}
+
+// Two neighbouring nodes (u0..u4 and u1..u5) of two variables in the
+// reference's form, each bit for bit weno5x2: the differences, their scaled
+// differences and six instead of ten loads are shared (71 packed operations
+// instead of 78).
+__device__ __forceinline__ float2 weno5x2_tail(float2 u1, float2 u2, float2 u3, float2 D12, float2 D23, float2 a0,
+                                               float2 a1, float2 a2, float2 ca0, float2 ca1, float2 ca2) {
+  const float2 eps = f2_(4.0e-6f);
+  const float2 b0 = __ffma2_rn(f2_(2.0f), D12, a0);
+  const float2 b1 = __fadd2_rn(u1, u3);
+  const float2 b2 = __ffma2_rn(f2_(-2.0f), D23, a2);
+  const float2 e0 = __ffma2_rn(ca0, a0, __ffma2_rn(b0, b0, eps));
+  const float2 e1 = __ffma2_rn(ca1, a1, __ffma2_rn(b1, b1, eps));
+  const float2 e2 = __ffma2_rn(ca2, a2, __ffma2_rn(b2, b2, eps));
+  const float2 d0 = __fmul2_rn(e0, e0), d1 = __fmul2_rn(e1, e1), d2 = __fmul2_rn(e2, e2);
+  const float2 P0 = __fmul2_rn(d1, d2);
+  const float2 P1 = __fmul2_rn(d0, d2);
+  const float2 P2 = __fmul2_rn(__fmul2_rn(f2_(0.5f), d0), d1);
+  const float2 s0 = __ffma2_rn(f2_(1.0f / 3.0f), b0, __fmul2_rn(f2_(-1.0f / 6.0f), D12));
+  const float2 S1 = __ffma2_rn(f2_(2.0f), D23, D12);
+  const float2 S2 = __ffma2_rn(f2_(-1.0f), b2, D23);
+  const float2 num = __ffma2_rn(P0, s0, __ffma2_rn(P1, S1, __fmul2_rn(P2, S2)));
+  const float2 den = __ffma2_rn(f2_(6.0f), __fadd2_rn(P1, P2), P0);
+  return __ffma2_rn(num, make_float2(rcp_(den.x), rcp_(den.y)), u2);
+}
+__device__ __forceinline__ void weno5x2_pair(float2 u0, float2 u1, float2 u2, float2 u3, float2 u4, float2 u5,
+                                             float2& a, float2& b) {
+  const float2 m1 = f2_(-1.0f), c = f2_(13.0f / 3.0f);
+  const float2 D01 = __ffma2_rn(m1, u0, u1), D12 = __ffma2_rn(m1, u1, u2), D23 = __ffma2_rn(m1, u2, u3);
+  const float2 D34 = __ffma2_rn(m1, u3, u4), D45 = __ffma2_rn(m1, u4, u5);
+  const float2 a0 = __ffma2_rn(m1, D01, D12), a1 = __ffma2_rn(m1, D12, D23), a2 = __ffma2_rn(m1, D23, D34);
+  const float2 a3 = __ffma2_rn(m1, D34, D45);
+  const float2 ca1 = __fmul2_rn(c, a1), ca2 = __fmul2_rn(c, a2);
+  a = weno5x2_tail(u1, u2, u3, D12, D23, a0, a1, a2, __fmul2_rn(c, a0), ca1, ca2);
+  b = weno5x2_tail(u2, u3, u4, D23, D34, a1, a2, a3, ca1, ca2, __fmul2_rn(c, a3));
 }
 
 // Both sides of two variables at once (published scheme): left[] as
