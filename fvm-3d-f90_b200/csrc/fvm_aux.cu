@@ -224,6 +224,21 @@ cudaError_t launch_fast_math_probe(const double* x, int64_t n, double* r, double
   return cudaGetLastError();
 }
 
+// The exact form's shared-denominator quotients x[i] / y[i] (a test hook).
+__global__ void exact_div_probe_kernel(const double* x, const double* y, int64_t n, double* q) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    double t[1] = {x[i]};
+    div_by_(t, recip_(y[i]));
+    q[i] = t[0];
+  }
+}
+
+cudaError_t launch_exact_div_probe(const double* x, const double* y, int64_t n, double* q, cudaStream_t s) {
+  if (n <= 0) return cudaSuccess;
+  exact_div_probe_kernel<<<grid_for(n, 256), 256, 0, s>>>(x, y, n, q);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_visc(const DevBlock* blocks, const DevCase* cases, const Task* tasks, int ntasks, int idim,
                         int prec, int role, cudaStream_t s, bool pdl) {
   if (prec == PREC_EXACT) return launch_visc_prec<PREC_EXACT>(blocks, cases, tasks, ntasks, idim, role, s, pdl);

@@ -58,6 +58,8 @@ cudaError_t launch_visc_fast(const DevBlock* blocks, const DevCase* cases, const
 cudaError_t visc_occupancy_fast(int prec, int* ctas_per_sm);
 // rcp_ / rsqrt_ of the non-exact FP64 forms over x[0..n) (device arrays).
 cudaError_t launch_fast_math_probe(const double* x, int64_t n, double* r, double* rs, cudaStream_t s);
+// x[i] / y[i] by the exact form's shared-denominator quotient (device arrays).
+cudaError_t launch_exact_div_probe(const double* x, const double* y, int64_t n, double* q, cudaStream_t s);
 
 // One compiled instantiation of the fused stage kernel.
 struct StageKernelInfo {

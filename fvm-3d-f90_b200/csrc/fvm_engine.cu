@@ -2055,6 +2055,20 @@ int fvm_test_drop_tensor_copies(fvm_ctx* ctx, int on) {
   return ctx->eng.set_drop_copies(on != 0);
 }
 
+int fvm_test_exact_div(const double* x, const double* y, int64_t n, double* q) {
+  if (!x || !y || !q || n < 0) return FVM_ERR_INVALID;
+  if (n == 0) return FVM_OK;
+  const size_t bytes = sizeof(double) * (size_t)n;
+  double* d = nullptr;
+  if (cudaMalloc(&d, 3 * bytes) != cudaSuccess) return FVM_ERR_CUDA;
+  cudaError_t e = cudaMemcpy(d, x, bytes, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(d + n, y, bytes, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = fvm::launch_exact_div_probe(d, d + n, n, d + 2 * n, 0);
+  if (e == cudaSuccess) e = cudaMemcpy(q, d + 2 * n, bytes, cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  return e == cudaSuccess ? FVM_OK : FVM_ERR_CUDA;
+}
+
 int fvm_test_fast_math(const double* x, int64_t n, double* rcp_out, double* rsqrt_out) {
   if (!x || !rcp_out || !rsqrt_out || n < 0) return FVM_ERR_INVALID;
   if (n == 0) return FVM_OK;

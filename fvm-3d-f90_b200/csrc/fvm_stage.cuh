@@ -244,14 +244,14 @@ __device__ __forceinline__ void cpy8(double* dst_smem, const double* src) {
 // Stencil value stored for reconstruction: conservative for WENO (the
 // reference reconstructs q, scheme_WENO.f90:28-72), primitive otherwise
 // (MUSCL / simple reconstruct p, scheme_reconstruct_MUSCL.f90:47-104).
-template <int RECON, class R, bool EX>
+template <int RECON, class R, bool EX, int DIM>
 __device__ __forceinline__ void to_stencil(const double q[5], R s[5], double gm1d, R gm1) {
   if constexpr (RECON == RECON_WENO_) {
 #pragma unroll
     for (int v = 0; v < 5; ++v) s[v] = (R)q[v];
   } else {
     if constexpr (sizeof(R) == 8) {
-      Prim5<double> p = cons2prim<double, EX>(q[0], q[1], q[2], q[3], q[4], gm1d);
+      Prim5<double> p = cons2prim<double, EX, EX && DIM == 2>(q[0], q[1], q[2], q[3], q[4], gm1d);
       s[0] = p.r; s[1] = p.u; s[2] = p.v; s[3] = p.w; s[4] = p.p;
     } else {
       Prim5<R> p = cons2prim<R, false>((R)q[0], (R)q[1], (R)q[2], (R)q[3], (R)q[4], gm1);
@@ -401,6 +401,7 @@ __device__ __forceinline__ void stage_run(const StageArgs& a) {
   double* sTZ = sTP + C::TPB;                                         // TMA: [5][TY][TX] z window's next plane
   __shared__ double s_red[6 * (NT / 32)];
   __shared__ int s_task;
+  __shared__ Recip s_rdr[3];  // EX: the cell sizes as denominators
   __shared__ __align__(8) uint64_t s_mbar[3];  // TMA: plane box, z box, RK operands
   __shared__ uint64_t s_issued;                  // TMA: globaltimer when this plane's copies were issued
   __shared__ uint64_t s_issp;                    // BOXA: globaltimer when the plane box was issued
@@ -474,6 +475,7 @@ __device__ __forceinline__ void stage_run(const StageArgs& a) {
     G.sy = B.sy; G.sz = B.sz; G.mask = B.ghost_mask;
     const double dr0 = B.dr[0], dr1 = B.dr[1], dr2 = B.dr[2];
     const double idr0 = B.inv_dr[0], idr1 = B.inv_dr[1], idr2 = B.inv_dr[2];
+    if (EX && tid < 3) s_rdr[tid] = recip_(B.dr[tid]);  // read in phase C, barriers later
     const double drv[3] = {dr0, dr1, dr2};
     const double idrv[3] = {idr0, idr1, idr2};
     const int rk_stages = CS.rk_stages, ts_set = CS.timestep_set, idim = CS.idim;
@@ -556,7 +558,7 @@ __device__ __forceinline__ void stage_run(const StageArgs& a) {
       for (int s = 0; s < C::WIN; ++s) {
         double q[5];
         ld5(qin, (int64_t)cxy + (int64_t)z_clamp(G, kstart - 1 + s) * G.sz, vs, q);
-        to_stencil<RECON, R, EX>(q, zw[s], gm1d, K.gm1);
+        to_stencil<RECON, R, EX, DIM>(q, zw[s], gm1d, K.gm1);
       }
     } else {
       // 2D: plane z0 into shared memory up front
@@ -566,7 +568,7 @@ __device__ __forceinline__ void stage_run(const StageArgs& a) {
           double q[5];
           R s[5];
           ld5(qin, (int64_t)lxy[sidx] + (int64_t)T.z0 * G.sz, vs, q);
-          to_stencil<RECON, R, EX>(q, s, gm1d, K.gm1);
+          to_stencil<RECON, R, EX, DIM>(q, s, gm1d, K.gm1);
 #pragma unroll
           for (int v = 0; v < 5; ++v) sP[v * PLANE + lsp[sidx]] = s[v];
         }
@@ -1198,6 +1200,26 @@ __device__ __forceinline__ void stage_run(const StageArgs& a) {
         const int fyl = C::NXF + ty * TX + tx;
         const int64_t off = off_k;
         double rhs[5];
+        if constexpr (EX) {
+          double t[5];
+#pragma unroll
+          for (int v = 0; v < 5; ++v) t[v] = (double)sF[v * NF + fxl + 1] - (double)sF[v * NF + fxl];
+          div_by_(t, s_rdr[0]);
+#pragma unroll
+          for (int v = 0; v < 5; ++v) rhs[v] = 0.0 - t[v];
+#pragma unroll
+          for (int v = 0; v < 5; ++v) t[v] = (double)sF[v * NF + fyl + TX] - (double)sF[v * NF + fyl];
+          div_by_(t, s_rdr[1]);
+#pragma unroll
+          for (int v = 0; v < 5; ++v) rhs[v] = rhs[v] - t[v];
+          if constexpr (DIM == 3) {
+#pragma unroll
+            for (int v = 0; v < 5; ++v) t[v] = (double)zF[v] - (double)zFprev[v];
+            div_by_(t, s_rdr[2]);
+#pragma unroll
+            for (int v = 0; v < 5; ++v) rhs[v] = rhs[v] - t[v];
+          }
+        } else
 #pragma unroll
         for (int v = 0; v < 5; ++v) {
           if constexpr (sizeof(R) == 4) {
@@ -1210,16 +1232,9 @@ __device__ __forceinline__ void stage_run(const StageArgs& a) {
           }
           const double fxr = (double)sF[v * NF + fxl + 1], fxL = (double)sF[v * NF + fxl];
           const double fyr = (double)sF[v * NF + fyl + TX], fyL = (double)sF[v * NF + fyl];
-          double r;
-          if constexpr (EX) {
-            r = 0.0 - (fxr - fxL) / dr0;
-            r = r - (fyr - fyL) / dr1;
-            if constexpr (DIM == 3) r = r - ((double)zF[v] - (double)zFprev[v]) / dr2;
-          } else {
-            r = -(fxr - fxL) * idr0;
-            r = r - (fyr - fyL) * idr1;
-            if constexpr (DIM == 3) r = r - ((double)zF[v] - (double)zFprev[v]) * idr2;
-          }
+          double r = -(fxr - fxL) * idr0;
+          r = r - (fyr - fyL) * idr1;
+          if constexpr (DIM == 3) r = r - ((double)zF[v] - (double)zFprev[v]) * idr2;
           rhs[v] = r;
         }
         if (visc) {
@@ -1320,7 +1335,7 @@ __device__ __forceinline__ void stage_run(const StageArgs& a) {
 #pragma unroll
             for (int v = 0; v < 5; ++v) zpre[v] = sZ[v * NC + tid];
           }
-          to_stencil<RECON, R, EX>(zpre, zw[C::WIN - 1], gm1d, K.gm1);
+          to_stencil<RECON, R, EX, DIM>(zpre, zw[C::WIN - 1], gm1d, K.gm1);
         }
         if (more_xy && !C::BOXA) {
           // centre of plane k+1 is window slot 1 after the shift
@@ -1345,7 +1360,7 @@ __device__ __forceinline__ void stage_run(const StageArgs& a) {
               for (int v = 0; v < 5; ++v) q[v] = pre[sidx][v];
             }
             R s[5];
-            to_stencil<RECON, R, EX>(q, s, gm1d, K.gm1);
+            to_stencil<RECON, R, EX, DIM>(q, s, gm1d, K.gm1);
 #pragma unroll
             for (int v = 0; v < 5; ++v) sP[v * PLANE + lsp[sidx]] = s[v];
           }

@@ -271,6 +271,10 @@ int fvm_test_drop_tensor_copies(fvm_ctx* ctx, int on);
  * counterpart in the reference. Evaluates both over the host array x[0..n)
  * on the device into host arrays rcp_out / rsqrt_out. */
 int fvm_test_fast_math(const double* x, int64_t n, double* rcp_out, double* rsqrt_out);
+/* Test hook of the exact form's quotients by a shared denominator; no
+ * counterpart in the reference. q[i] = x[i] / y[i] over host arrays, which the
+ * method must round as the division does. */
+int fvm_test_exact_div(const double* x, const double* y, int64_t n, double* q);
 
 /* Residual norms of one block's rhs in device memory, as
  * ClassIteration%compute_residual_sub (class_iteration.f90, file-local
