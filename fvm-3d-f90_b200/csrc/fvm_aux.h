@@ -36,8 +36,11 @@ cudaError_t launch_unpack(double* role_blk, int64_t vs, int sy, int sz, int ni, 
                           cudaStream_t s);
 cudaError_t launch_pack(const double* role_blk, int64_t vs, int sy, int sz, int ni, int nj, int nk, double* dst,
                         int prim, double gm1, cudaStream_t s);
-cudaError_t launch_init_dt(const DevBlock* blocks, int nblocks, const DevCase* cases, DevCaseState* st, int ncases,
-                           unsigned long long* case_max, const int* mask, int role, cudaStream_t s);
+// dt of the cases in mask from the state in `role`; max_cells: cells of the
+// largest block.
+cudaError_t launch_init_dt(const DevBlock* blocks, int nblocks, int64_t max_cells, const DevCase* cases,
+                           DevCaseState* st, int ncases, unsigned long long* case_max, const int* mask, int role,
+                           cudaStream_t s);
 cudaError_t launch_finalize(const DevBlock* blocks, const DevCase* cases, const int* case_blk, DevCaseState* st,
                             int ncases, const double* partials, int* counters, int ncounters, cudaStream_t s,
                             bool pdl = false);

@@ -1546,7 +1546,10 @@ int Engine::prepare() {
       dtmask_cap_ = (int)cases.size();
     }
     CK(cudaMemcpyAsync(d_dtmask_, mask.data(), sizeof(int) * cases.size(), cudaMemcpyHostToDevice, stream));
-    CK(launch_init_dt(d_blocks_, (int)blocks.size(), d_cases_, d_state_, (int)cases.size(), d_casemax_, d_dtmask_,
+    int64_t max_cells = 0;
+    for (const auto& b : blocks)
+      if (!b.dead) max_cells = std::max(max_cells, b.n[0] * b.n[1] * b.n[2]);
+    CK(launch_init_dt(d_blocks_, (int)blocks.size(), max_cells, d_cases_, d_state_, (int)cases.size(), d_casemax_, d_dtmask_,
                       ROLE_A, stream));
     CK(cudaStreamSynchronize(stream));  // the mask's host copy goes out of scope
     for (auto& c : cases) c.dt_stale = false;
