@@ -1383,7 +1383,29 @@ int Engine::enqueue_step(cudaEvent_t* evs, int nev, int* kinds, int* nlaunch) {
   };
   if (evs && nev > 0) CK(cudaEventRecord(evs[0], stream));
   int ev_i = 0;
-  for (int m = 1; m <= S; ++m) {
+  // Groups that share no launch between their stages (no ghost gather, no
+  // viscous kernel) run the whole step as one branch each and join once, at the
+  // finalize: joining after every stage leaves the GPU to the slowest group
+  // three times a step (24 mixed FP32 cases 1069 -> 1055 us per step).
+  bool apart = fork && npairs == 0;
+  for (int li = 0; li < 6; ++li) apart = apart && vlist_n_[li] == 0;
+  if (apart) {
+    CK(cudaEventRecord(fork_ev_[0], stream));
+    for (size_t g = 0; g < groups.size(); ++g) {
+      const Group& G = groups[g];
+      CK(cudaStreamWaitEvent(side_[g], fork_ev_[0], 0));
+      for (int m = 1; m <= S; ++m) {
+        StageArgs a = stage_args((int)g, m);
+        void* args[] = {&a};
+        LaunchCfg L(dim3(G.grid), dim3(G.k.threads), G.k.smem, side_[g], m > 1);
+        CK(cudaLaunchKernelExC(&L.cfg, G.k.fn, args));
+        CK(mark(1));
+      }
+      CK(cudaEventRecord(fork_ev_[g + 1], side_[g]));
+      CK(cudaStreamWaitEvent(stream, fork_ev_[g + 1], 0));
+    }
+  }
+  for (int m = 1; m <= S && !apart; ++m) {
     int rin, rout;
     stage_roles(S, m, &rin, &rout);
     for (int li = 0; li < 6; ++li) {
