@@ -110,20 +110,6 @@ double even_split(const std::vector<ZColumn>& cols, int slots, double ovh, std::
   return share;
 }
 
-// Makespan of the persistent work queue for tasks of the given costs on
-// `slots` CTAs: tasks are taken longest first, each by the CTA that frees
-// first (what the atomic task counter does when costs are uniform per plane).
-double queue_makespan(std::vector<double>& cost, int slots) {
-  std::sort(cost.begin(), cost.end(), std::greater<double>());
-  std::vector<double> heap(std::max(1, slots), 0.0);  // min-heap of finish times
-  auto cmp = std::greater<double>();
-  for (double c : cost) {
-    std::pop_heap(heap.begin(), heap.end(), cmp);
-    heap.back() += c;
-    std::push_heap(heap.begin(), heap.end(), cmp);
-  }
-  return *std::max_element(heap.begin(), heap.end());
-}
 inline int stage_roles(int S, int m, int* rin, int* rout) {
   // RK3: A->B, (A,B)->C, (A,C)->A. RK4: A->B, B->C, C->B, B->A (q0 = A).
   static const int r3[3][2] = {{ROLE_A, ROLE_B}, {ROLE_B, ROLE_C}, {ROLE_C, ROLE_A}};
@@ -945,13 +931,13 @@ int Engine::plan() {
   ntasks_total = (int64_t)tasks.size();
 
   // -- viscous task lists, one per (precision form, dimension): Navier-Stokes
-  // blocks in column tiles over equal z chunks. The kernel is
-  // throughput-bound per SM (its CTAs share the SM's shared-memory pipe), so
-  // a 3D chunk length is scored by the largest per-SM sum of task costs
-  // (longest-first onto the SMs) over the CTAs an SM holds, but no less than
-  // half the longest task (an SM left with one task runs it at most about
-  // twice as fast). A task of c planes costs c plane-times plus its prologue
-  // (two extra planes converted, one extra z face).
+  // blocks in column tiles, in 3D split evenly over the CTAs an SM holds (a
+  // piece's prologue converts two extra planes and computes one extra z face,
+  // about 1.5 planes), longest first; two rounds of shares in the FP32 form,
+  // whose CTAs are six to an SM. Per step, against equal chunks picked by a
+  // per-SM makespan estimate: Taylor-Green 75^3 FP32 249 -> 220 us, 110^3 FP32
+  // 577 -> 489, 50^3 exact 504 -> 431, 128^3 FP64 825 -> 816 (two rounds 823;
+  // FP32 75^3 with one round 223, 110^3 518).
   for (int prec = 0; prec < 3; ++prec) {
     for (int dim : {3, 2}) {
       const int li = prec * 2 + (dim == 3 ? 0 : 1);
@@ -963,50 +949,22 @@ int Engine::plan() {
         if (c.equation == FVM_EQ_NAVIER_STOKES && c.idimension == dim && c.precision == prec)
           ns.push_back(&blocks[bi]);
       }
-      int64_t vz = 16;
-      std::vector<int64_t> z0s;
       if (dim == 3 && !ns.empty()) {
         int occ = 1;
         CK(visc_occupancy(prec, &occ));
-        double best = 0.0;
-        std::vector<double> cost;
-        for (int64_t cand = 64; cand >= 4; cand -= (cand > 16 ? 4 : 2)) {
-          cost.clear();
-          double longest = 0.0;
-          for (const HBlock* b : ns) {
-            const int64_t ncol = ((b->n[0] + vtx - 1) / vtx) * ((b->n[1] + vty - 1) / vty);
-            equal_chunks(b->n[2], cand, z0s);
-            for (size_t c = 0; c + 1 < z0s.size(); ++c)
-              for (int64_t q = 0; q < ncol; ++q) {
-                cost.push_back((double)(z0s[c + 1] - z0s[c]) + 1.5);
-                longest = std::max(longest, cost.back());
-              }
-          }
-          const double m = std::max(queue_makespan(cost, num_sms) / occ, 0.5 * longest);
-          if (best <= 0.0 || m < best * 0.995) {
-            best = m;
-            vz = cand;
-          }
-        }
-      }
-      for (const HBlock* b : ns) {
-        const int bi = (int)(b - blocks.data());
-        if (dim == 3)
-          equal_chunks(b->n[2], vz, z0s);
-        else
-          z0s = {0, b->n[2]};
-        for (size_t ch = 0; ch + 1 < z0s.size(); ++ch)
+        std::vector<ZColumn> cols;
+        for (const HBlock* b : ns)
           for (int64_t y0 = 0; y0 < b->n[1]; y0 += vty)
-            for (int64_t x0 = 0; x0 < b->n[0]; x0 += vtx) {
-              Task t;
-              t.blk = bi;
-              t.x0 = (int)x0;
-              t.y0 = (int)y0;
-              t.z0 = (int)z0s[ch];
-              t.z1 = (int)z0s[ch + 1];
-              t.slot = 0;
-              tasks.push_back(t);
-            }
+            for (int64_t x0 = 0; x0 < b->n[0]; x0 += vtx)
+              cols.push_back({(int)(b - blocks.data()), (int)x0, (int)y0, (int)b->n[2]});
+        even_split(cols, occ * num_sms * (prec == FVM_PREC_FP32_FLUX ? 2 : 1), 1.5, tasks);
+        std::stable_sort(tasks.begin() + vlist_off_[li], tasks.end(),
+                         [](const Task& a, const Task& b) { return (a.z1 - a.z0) > (b.z1 - b.z0); });
+      } else {
+        for (const HBlock* b : ns)
+          for (int64_t y0 = 0; y0 < b->n[1]; y0 += vty)
+            for (int64_t x0 = 0; x0 < b->n[0]; x0 += vtx)
+              tasks.push_back({(int)(b - blocks.data()), (int)x0, (int)y0, 0, (int)b->n[2], 0});
       }
       vlist_n_[li] = (int)tasks.size() - vlist_off_[li];
     }

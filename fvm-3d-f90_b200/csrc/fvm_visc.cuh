@@ -343,9 +343,9 @@ __device__ __forceinline__ void visc_tile_body(const DevBlock& B, const DevCase&
           if (IDIM == 3) V[v] = V[v] + (Gzr[v] - Gzl[v]) * idr[2];
         }
       }
-      V[0] = R(0);
       const int64_t o = (T.x0 + tx) + (int64_t)(T.y0 + ty) * B.sy + (int64_t)k * B.sz;
-      for (int v = 0; v < 5; ++v) B.visc[o + v * vs] = (double)V[v];
+      // (V[0] is zero: neither written nor read)
+      for (int v = 1; v < 5; ++v) B.visc[o + v * vs] = (double)V[v];
     }
     if (IDIM == 3) {
 #pragma unroll
