@@ -1239,7 +1239,7 @@ __device__ __forceinline__ void stage_run(const StageArgs& a) {
         }
         if (visc) {
 #pragma unroll
-          for (int v = 1; v < 5; ++v) rhs[v] = rhs[v] + visc[off + v * vs];
+          for (int v = 0; v < 5; ++v) rhs[v] = rhs[v] + visc[off + v * vs];
         }
         // RK update (scheme_Runge_Kutta.f90:30-63; classic RK4 for 4 stages)
         double u0[5], um[5], ac[5];
