@@ -892,7 +892,17 @@ int Engine::plan() {
     }
     if (!cols.empty()) {
       const size_t first = gt.size();
-      const double share = even_split(cols, G.grid, ovh, gt);
+      double share = even_split(cols, G.grid, ovh, gt);
+      // One round of shares is best (two: vortex 128^3 FP64 841 -> 870 us, 61x83x47
+      // blast 131 -> 142, 160^3 FP32 1009 -> 1035) until the FP64 forms' shares
+      // are so long that the CTAs drift apart by more than a second piece's
+      // warm-up costs: 64 planes (160^3 published form 1983 -> 1941), 16 in the
+      // exact form, whose planes take three times as long (vortex 100^3 2041 ->
+      // 1897).
+      if (G.prec != FVM_PREC_FP32_FLUX && share >= (G.prec == FVM_PREC_FP64_EXACT ? 16.0 : 64.0)) {
+        gt.resize(first);
+        share = even_split(cols, 2 * G.grid, ovh, gt);
+      }
       // The FP32 form reads its tile halos at a third of the HBM rate, so it
       // gains from neighbouring columns marching in step (their halos meet in
       // L2): equal chunks that fit one round and come within 8 % of the even
