@@ -67,6 +67,10 @@ __device__ __forceinline__ double nsqrt_(double x) { return x * rsqrt_(x); }
 __device__ __forceinline__ float nsqrt_(float x) { return sqrtf(x); }
 __device__ __forceinline__ double abs_(double x) { return fabs(x); }
 __device__ __forceinline__ float abs_(float x) { return fabsf(x); }
+// 2^-e for x = +-1.f 2^e, so that |x pow2_inv_(x)| is in [1, 2).
+__device__ __forceinline__ double pow2_inv_(double x) {
+  return __hiloint2double(0x7fe00000 - (__double2hiint(x) & 0x7ff00000), 0);
+}
 __device__ __forceinline__ double sgn1_(double x) { return copysign(1.0, x); }
 __device__ __forceinline__ float sgn1_(float x) { return copysignf(1.0f, x); }
 template <class R> __device__ __forceinline__ R min2_(R a, R b) { return (b < a) ? b : a; }
@@ -804,17 +808,23 @@ __device__ __forceinline__ void flux_ausm(const Prim5<R>& L, const Prim5<R>& Rs,
     M_l = Vc_l / c_l;
     M_r = Vc_r / c_r;
   } else if constexpr (sizeof(R) == 8) {
-    // one reciprocal square root t of gamma p rho per side: rho c = gamma p
-    // rho t, 1 / c = rho t, 1 / rho = gamma p t^2 (c_l, c_r hold rho c)
-    const R gl = k.gamma * L.p, gr = k.gamma * Rs.p;
-    const R xl = gl * L.r, xr = gr * Rs.r;
-    const R tl = rsqrt_(xl), tr = rsqrt_(xr);
-    c_l = copysign(xl * tl, L.r);
-    c_r = copysign(xr * tr, Rs.r);
-    M_l = Vc_l * (abs_(L.r) * tl);
-    M_r = Vc_r * (abs_(Rs.r) * tr);
-    H_l = (k.goverg1 * L.p) * (gl * (tl * tl)) + R(0.5) * (L.u * L.u + L.v * L.v + L.w * L.w);
-    H_r = (k.goverg1 * Rs.p) * (gr * (tr * tr)) + R(0.5) * (Rs.u * Rs.u + Rs.v * Rs.v + Rs.w * Rs.w);
+    // One reciprocal square root per side. With s = 2^-exponent(rho), m = rho s
+    // and g = gamma p s (both scalings are exact), t = (g m)^(-1/2) gives
+    // 1 / c = |m| t, c = g t and p / rho = p s (c t), and no product leaves the
+    // range where p / rho does not (gamma p rho alone would: 2 FP64 operations
+    // a side less, and NaN where density and pressure are both below 1e-154).
+    // c_l and c_r hold rho c.
+    const R sl = pow2_inv_(L.r), sr = pow2_inv_(Rs.r);
+    const R ml = L.r * sl, mr = Rs.r * sr, pl = L.p * sl, pr = Rs.p * sr;
+    const R gl = k.gamma * pl, gr = k.gamma * pr;
+    const R tl = rsqrt_(gl * ml), tr = rsqrt_(gr * mr);
+    const R cl = gl * tl, cr = gr * tr;
+    c_l = abs_(L.r) * cl;
+    c_r = abs_(Rs.r) * cr;
+    M_l = Vc_l * (abs_(ml) * tl);
+    M_r = Vc_r * (abs_(mr) * tr);
+    H_l = (k.goverg1 * pl) * (cl * tl) + R(0.5) * (L.u * L.u + L.v * L.v + L.w * L.w);
+    H_r = (k.goverg1 * pr) * (cr * tr) + R(0.5) * (Rs.u * Rs.u + Rs.v * Rs.v + Rs.w * Rs.w);
   } else {
     const R irl = rcp_(L.r), irr = rcp_(Rs.r);
     const R pl = L.p * irl, pr = Rs.p * irr;
