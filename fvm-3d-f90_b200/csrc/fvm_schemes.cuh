@@ -214,6 +214,15 @@ __device__ __forceinline__ void muscl_slopes(R p1, R p2, R p3, int lim, R& Dbm, 
   }
 }
 
+// x, or NaN where a or b is one. One comparison and one select of the high word
+// (two isnan tests and a select of both words: 2D Riemann 700^2 142.0 -> 144.3 us
+// per step).
+__device__ __forceinline__ double nan_where_unordered_(double x, double a, double b) {
+  int h = __double2hiint(x);
+  asm("{.reg .pred p; setp.nan.f64 p, %1, %2; selp.b32 %0, 0x7fffffff, %0, p;}" : "+r"(h) : "d"(a), "d"(b));
+  return __hiloint2double(h, __double2loint(x));
+}
+
 // The non-exact FP64 node: the values qr, ql of centre p2 at its right and left
 // faces. The three limiters give one slope for both faces (minmod with b = 1
 // is symmetric), and (1 - kappa) + (1 + kappa) = 2, so the faces are p2 +- D/2
@@ -227,8 +236,10 @@ __device__ __forceinline__ void muscl_node_fp64(double p1, double p2, double p3,
   const double Dm = p2 - p1, Dp = p3 - p2;
   double D;
   if constexpr (LIM == LIM_MINMOD_) {
-    const double pr = Dm * Dp, m = abs_(Dp) < abs_(Dm) ? Dp : Dm;
-    D = pr > 0.0 ? m : (pr <= 0.0 ? 0.0 : pr);  // the last: NaN
+    // The signs decide, not the product's, which underflows to zero where the
+    // differences do not.
+    const bool opposite = (__double2hiint(Dm) ^ __double2hiint(Dp)) < 0;
+    D = nan_where_unordered_(opposite ? 0.0 : (abs_(Dp) < abs_(Dm) ? Dp : Dm), Dm, Dp);
   } else if constexpr (LIM == LIM_VANLEER_) {
     // (sign Dm + sign Dp) Dm Dp / (|Dm| + |Dp| + e): opposite signs give 0
     const double s = (__double2hiint(Dm) ^ __double2hiint(Dp)) < 0 ? 0.0 : copysign(2.0, Dm);

@@ -40,3 +40,15 @@ def test_ausm_where_density_times_pressure_leaves_the_range(recon, exp):
     ref, got = evolve(0, abi.PREC_FP64, **cfg), evolve(exp, abi.PREC_FP64, **cfg)
     assert np.isfinite(ref).all() and np.isfinite(got).all()
     assert np.abs(got - ref).max() <= 1e-12 * np.abs(ref).max()
+
+
+# Differences of neighbouring cells of 1e-160 have a product that underflows;
+# minmod compares magnitudes and signs and does not multiply. Every operation
+# of this sweep scales exactly.
+@pytest.mark.parametrize("prec", [abi.PREC_FP64_EXACT, abi.PREC_FP64])
+def test_minmod_slopes_of_small_differences(prec):
+    cfg = dict(reconstruct=abi.RECON_MUSCL, limiter=abi.LIMITER_MINMOD, kappa=1.0 / 3.0,
+               flux_split=abi.FLUX_VANLEER)
+    ref, got = evolve(0, prec, **cfg), evolve(-560, prec, **cfg)
+    assert np.isfinite(ref).all()
+    assert np.array_equal(got, ref)
