@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "fvm_engine.h"
+#include "fvm_split.h"
 
 #include <cudaTypedefs.h>  // PFN_cuTensorMapEncodeTiled
 
@@ -36,78 +37,6 @@ PFN_cuTensorMapEncodeTiled encode_fn() {
       fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled>(p);
   }
   return fn;
-}
-
-// Split nz planes into chunks of at most L planes, all of nearly equal length
-// (lengths differ by at most one plane).
-inline void equal_chunks(int64_t nz, int64_t L, std::vector<int64_t>& z0s) {
-  z0s.clear();
-  const int64_t nc = std::max<int64_t>(1, (nz + L - 1) / L);
-  const int64_t base = nz / nc, extra = nz % nc;
-  int64_t z = 0;
-  for (int64_t c = 0; c < nc; ++c) {
-    z0s.push_back(z);
-    z += base + (c < extra ? 1 : 0);
-  }
-  z0s.push_back(nz);
-}
-
-// A z column of one tile.
-struct ZColumn {
-  int blk, x0, y0, nz;
-};
-
-// Cut the columns into equal chunks of at most L planes.
-void chunk_columns(const std::vector<ZColumn>& cols, int64_t L, std::vector<Task>& out) {
-  std::vector<int64_t> z0s;
-  for (const auto& c : cols) {
-    equal_chunks(c.nz, L, z0s);
-    for (size_t i = 0; i + 1 < z0s.size(); ++i) out.push_back({c.blk, c.x0, c.y0, (int)z0s[i], (int)z0s[i + 1], 0});
-  }
-}
-
-// Even split of z columns over `slots` resident CTAs: the columns, taken one
-// after the other, are cut wherever a CTA's share of the work is full, so all
-// shares are the same to within a plane or two and a stage is one round of the
-// queue (equal chunks leave CTAs idle in its last round: 2.3 rounds on the
-// 128^3 vortex, 0.8 of one on a 61x83x47 blast). A piece of c planes costs
-// c + ovh plane-times (the z window's warm-up and the set-up) and has at least
-// kMinPiece planes where the column allows it. The smallest share that fits is
-// found by growing it from the mean: O(pieces) per try, a few tries, so the
-// re-plans of a serving loop stay cheap. Measured per step, equal chunks of
-// the length a queue estimate picked -> even split: vortex 128^3 FP64 926 ->
-// 909 us, 64^3 172 -> 153; Taylor-Green 128^3 FP64 877 -> 833, 30^3 FP32 96 ->
-// 74; 61x83x47 blast FP64 159 -> 138; 24 mixed FP32 cases 1143 -> 1086. The
-// pieces' least length (1 to 3) and ovh (0.6 to 1.4 for WENO) move these by
-// less than 2 %. Returns the share.
-double even_split(const std::vector<ZColumn>& cols, int slots, double ovh, std::vector<Task>& out) {
-  constexpr int kMinPiece = 2, kTries = 400;
-  double total = 0.0;
-  for (const auto& c : cols) total += c.nz;
-  const size_t first = out.size();
-  double share = std::max(total / slots, (double)kMinPiece) + ovh;
-  for (int it = 0; it < kTries; ++it, share += std::max(0.25, share / 128.0)) {
-    out.resize(first);
-    int used = 1;
-    double left = share;
-    for (const auto& c : cols) {
-      for (int z = 0; z < c.nz;) {
-        if (left < ovh + std::min(kMinPiece, c.nz - z)) {
-          ++used;
-          left = share;
-        }
-        int n = std::min(c.nz - z, std::max(kMinPiece, (int)(left - ovh)));
-        const int rest = c.nz - z - n;
-        if (rest > 0 && rest < kMinPiece) n += n >= 2 * kMinPiece - rest ? rest - kMinPiece : rest;
-        out.push_back({c.blk, c.x0, c.y0, z, z + n, 0});
-        z += n;
-        left -= n + ovh;
-      }
-      if (used > slots && it + 1 < kTries) break;  // does not fit: a larger share
-    }
-    if (used <= slots) break;
-  }
-  return share;
 }
 
 inline int stage_roles(int S, int m, int* rin, int* rout) {
@@ -890,38 +819,7 @@ int Engine::plan() {
       }
       gt.insert(gt.end(), ct.begin(), ct.end());
     }
-    if (!cols.empty()) {
-      const size_t first = gt.size();
-      double share = even_split(cols, G.grid, ovh, gt);
-      // One round of shares is best (two: vortex 128^3 FP64 841 -> 870 us, 61x83x47
-      // blast 131 -> 142, 160^3 FP32 1009 -> 1035) until the FP64 forms' shares
-      // are so long that the CTAs drift apart by more than a second piece's
-      // warm-up costs: 64 planes (160^3 published form 1983 -> 1941), 16 in the
-      // exact form, whose planes take three times as long (vortex 100^3 2041 ->
-      // 1897).
-      if (G.prec != FVM_PREC_FP32_FLUX && share >= (G.prec == FVM_PREC_FP64_EXACT ? 16.0 : 64.0)) {
-        gt.resize(first);
-        share = even_split(cols, 2 * G.grid, ovh, gt);
-      }
-      // The FP32 form reads its tile halos at a third of the HBM rate, so it
-      // gains from neighbouring columns marching in step (their halos meet in
-      // L2): equal chunks that fit one round and come within 8 % of the even
-      // share replace it (Taylor-Green 110^3 608 -> 592 us, 90^3 vortex 338 ->
-      // 332). The FP64 forms do not notice (112^3 blast 374 even, 412 chunked).
-      if (G.prec == FVM_PREC_FP32_FLUX) {
-        int64_t nz = 0;
-        for (const auto& c : cols) nz = std::max<int64_t>(nz, c.nz);
-        int64_t L = std::max<int64_t>(4, (int64_t)share - 1);
-        for (; L <= nz && (double)L + ovh <= 1.08 * share; ++L) {
-          int64_t n = 0;
-          for (const auto& c : cols) n += (c.nz + L - 1) / L;
-          if (n > G.grid) continue;
-          gt.resize(first);
-          chunk_columns(cols, L, gt);
-          break;
-        }
-      }
-    }
+    if (!cols.empty()) split_columns(cols, G.grid, G.prec, ovh, gt);
     std::stable_sort(gt.begin(), gt.end(), [](const Task& a, const Task& b) { return (a.z1 - a.z0) > (b.z1 - b.z0); });
     tasks.insert(tasks.end(), gt.begin(), gt.end());
     G.ntasks = (int)tasks.size() - G.task_off;
