@@ -109,7 +109,8 @@ def autotune(solver, ncells: int, zchunks=(0, 8, 16, 32, 64), tiles=(0, 1, 2, 3)
     three_d = solver.cfg.idimension == 3
     for t in tiles:
         for z in (zchunks if three_d else (0,)):
-            for sp in (splits if three_d else (1,)):
+            # the engine's own chunks (z = 0) have no tail to split
+            for sp in (splits if three_d and z > 0 else (1,)):
                 set_tuning(solver, 0, t, z)
                 set_tail_split(solver, 0, sp)
                 time_step(solver, 1)  # warm-up
