@@ -343,43 +343,45 @@ __device__ __forceinline__ double weno5_right(const WenoParts& w, double u2) {
   return fma(-num, rcp_twice_(fma(3.0, w.P0, fma(6.0, w.P1, w.P2))), u2);
 }
 
-// scheme_WENO.f90:87-121 (WENO_JS on u0..u4, value at the right face of u2).
-// textbook != 0: IS_1 with (u1-u3)^2 (Jiang & Shu); 0: (u1+u3)^2 as written.
-// TB: the non-exact form's choice of IS_1 at compile time.
-template <class R, bool EX, bool TB>
-__device__ __forceinline__ R weno5(R u0, R u1, R u2, R u3, R u4, int textbook) {
-  if constexpr (EX) {
-    const R q0 = R(1.0 / 3.0) * u0 - R(7.0 / 6.0) * u1 + R(11.0 / 6.0) * u2;
-    const R q1 = R(-1.0 / 6.0) * u1 + R(5.0 / 6.0) * u2 + R(1.0 / 3.0) * u3;
-    const R q2 = R(1.0 / 3.0) * u2 + R(5.0 / 6.0) * u3 - R(1.0 / 6.0) * u4;
-    const R a0 = u0 - R(2.0) * u1 + u2;
-    const R b0 = u0 - R(4.0) * u1 + R(3.0) * u2;
-    const R a1 = u1 - R(2.0) * u2 + u3;
-    const R b1 = textbook ? (u1 - u3) : (u1 + u3);
-    const R a2 = u2 - R(2.0) * u3 + u4;
-    const R b2 = R(3.0) * u2 - R(4.0) * u3 + u4;
-    const R IS0 = R(13.0 / 12.0) * (a0 * a0) + R(1.0 / 4.0) * (b0 * b0);
-    const R IS1 = R(13.0 / 12.0) * (a1 * a1) + R(1.0 / 4.0) * (b1 * b1);
-    const R IS2 = R(13.0 / 12.0) * (a2 * a2) + R(1.0 / 4.0) * (b2 * b2);
-    const R e0 = IS0 + R(1.0e-6), e1 = IS1 + R(1.0e-6), e2 = IS2 + R(1.0e-6);
-    const R al0 = R(0.1) / (e0 * e0);
-    const R al1 = R(0.6) / (e1 * e1);
-    const R al2 = R(0.3) / (e2 * e2);
-    const R as = al0 + al1 + al2;
-    double w[3] = {al0, al1, al2};
-    div_by_(w, recip_(as));
-    return w[0] * q0 + w[1] * q1 + w[2] * q2;
-  } else {
-    // The same mathematics in fewer operations (weno5_parts): the weights are
-    // division-free and the result is u2 + sum omega_k delta_k.
-    const WenoParts w = weno5_parts<TB>(u0, u1, u2, u3, u4);
-    return weno5_left(w, u2);
-  }
+// The exact form: scheme_WENO.f90:87-121 (WENO_JS on u0..u4, value at the right
+// face of u2). textbook != 0: IS_1 with (u1-u3)^2 (Jiang & Shu); 0: (u1+u3)^2
+// as written.
+template <class R>
+__device__ __forceinline__ R weno5_exact(R u0, R u1, R u2, R u3, R u4, int textbook) {
+  const R q0 = R(1.0 / 3.0) * u0 - R(7.0 / 6.0) * u1 + R(11.0 / 6.0) * u2;
+  const R q1 = R(-1.0 / 6.0) * u1 + R(5.0 / 6.0) * u2 + R(1.0 / 3.0) * u3;
+  const R q2 = R(1.0 / 3.0) * u2 + R(5.0 / 6.0) * u3 - R(1.0 / 6.0) * u4;
+  const R a0 = u0 - R(2.0) * u1 + u2;
+  const R b0 = u0 - R(4.0) * u1 + R(3.0) * u2;
+  const R a1 = u1 - R(2.0) * u2 + u3;
+  const R b1 = textbook ? (u1 - u3) : (u1 + u3);
+  const R a2 = u2 - R(2.0) * u3 + u4;
+  const R b2 = R(3.0) * u2 - R(4.0) * u3 + u4;
+  const R IS0 = R(13.0 / 12.0) * (a0 * a0) + R(1.0 / 4.0) * (b0 * b0);
+  const R IS1 = R(13.0 / 12.0) * (a1 * a1) + R(1.0 / 4.0) * (b1 * b1);
+  const R IS2 = R(13.0 / 12.0) * (a2 * a2) + R(1.0 / 4.0) * (b2 * b2);
+  const R e0 = IS0 + R(1.0e-6), e1 = IS1 + R(1.0e-6), e2 = IS2 + R(1.0e-6);
+  const R al0 = R(0.1) / (e0 * e0);
+  const R al1 = R(0.6) / (e1 * e1);
+  const R al2 = R(0.3) / (e2 * e2);
+  const R as = al0 + al1 + al2;
+  double w[3] = {al0, al1, al2};
+  div_by_(w, recip_(as));
+  return w[0] * q0 + w[1] * q1 + w[2] * q2;
 }
 
 // Two WENO5 evaluations at once in packed FP32 (sm_100 f32x2 FMA / add /
-// multiply: one instruction per pair), for the FP32 flux form: the
-// difference form of weno5<R, false>; the pair shares `textbook`.
+// multiply: one instruction per pair), for the FP32 flux form; the pair shares
+// `textbook`. With the first differences Dij = uj - ui the candidates are
+// q_k = u2 + delta_k (delta_0 = (5 D12 - 2 D01)/6, delta_1 = (D12 + 2 D23)/6,
+// delta_2 = (4 D23 - D34)/6); a_k are the second differences, b_0 = 2 D12 + a_0,
+// b_2 = a_2 - 2 D23. The smoothness indicators and eps are scaled by 4 (the
+// weights only see their ratios): 4 (IS_k + eps) = 13/3 a_k^2 + b_k^2 + 4e-6.
+// The weights are division-free, omega_k = c_k prod_{j!=k} d_j / D with
+// d = e^2: with P0 = d1 d2, P1 = d0 d2 and P2 = d0 d1 / 2 they are
+// (P0, 6 P1, 6 P2) / (P0 + 6 (P1 + P2)), so the constants of the linear weights
+// fold into 6 delta_1 = D12 + 2 D23 and 6 delta_2 = 4 D23 - D34 (one operation
+// each).
 __device__ __forceinline__ float2 f2_(float a) { return make_float2(a, a); }
 __device__ __forceinline__ float2 weno5x2(float2 u0, float2 u1, float2 u2, float2 u3, float2 u4, int textbook) {
   const float2 m1 = f2_(-1.0f);
@@ -395,12 +397,10 @@ __device__ __forceinline__ float2 weno5x2(float2 u0, float2 u1, float2 u2, float
   const float2 e1 = __ffma2_rn(__fmul2_rn(c, a1), a1, __ffma2_rn(b1, b1, eps));
   const float2 e2 = __ffma2_rn(__fmul2_rn(c, a2), a2, __ffma2_rn(b2, b2, eps));
   const float2 d0 = __fmul2_rn(e0, e0), d1 = __fmul2_rn(e1, e1), d2 = __fmul2_rn(e2, e2);
-  // weights c_k / d_k normalised by 1 / c_0, with the constants of c_1 and
-  // c_2 folded into the differences (the FP64 form's P0, P1, P2, S1, S2)
   const float2 P0 = __fmul2_rn(d1, d2);
   const float2 P1 = __fmul2_rn(d0, d2);
   const float2 P2 = __fmul2_rn(__fmul2_rn(f2_(0.5f), d0), d1);
-  const float2 s0 = __ffma2_rn(f2_(1.0f / 3.0f), b0, __fmul2_rn(f2_(-1.0f / 6.0f), D12));
+  const float2 s0 = __ffma2_rn(f2_(1.0f / 3.0f), b0, __fmul2_rn(f2_(-1.0f / 6.0f), D12));  // delta_0 = (2 b_0 - D12) / 6
   const float2 S1 = __ffma2_rn(f2_(2.0f), D23, D12);
   const float2 S2 = __ffma2_rn(m1, b2, D23);  // 4 D23 - D34
   const float2 num = __ffma2_rn(P0, s0, __ffma2_rn(P1, S1, __fmul2_rn(P2, S2)));
@@ -490,48 +490,38 @@ __device__ __forceinline__ void weno5x2_both(float2 u0, float2 u1, float2 u2, fl
 
 // The WENO node values of one stencil u[var][0..4]: wm (left-biased, value
 // at the right face of u[.][2]) and, with TB, wp (mirrored, value at its left
-// face, always the textbook form). The FP32 flux form evaluates them in pairs.
+// face, always the textbook form). The FP32 flux form comes here with TB only,
+// which TEXTBOOK compat implies; its left-biased nodes alone, like most of the
+// FP64 form's, are evaluated in neighbouring pairs by the stage kernel.
 template <class R, bool EX, bool TB>
 __device__ __forceinline__ void weno5_node(const R (&u)[5][5], int textbook, R wm[5], R wp[5]) {
   if constexpr (sizeof(R) == 4) {
-    if constexpr (TB) {
-      // TB implies TEXTBOOK compat, so both sides take the textbook form
+    static_assert(TB, "the stage kernel evaluates left-biased FP32 nodes itself");
 #pragma unroll
-      for (int v = 0; v < 4; v += 2) {
-        float2 l, r;
-        weno5x2_both(make_float2(u[v][0], u[v + 1][0]), make_float2(u[v][1], u[v + 1][1]),
-                     make_float2(u[v][2], u[v + 1][2]), make_float2(u[v][3], u[v + 1][3]),
-                     make_float2(u[v][4], u[v + 1][4]), l, r);
-        wm[v] = l.x;
-        wm[v + 1] = l.y;
-        wp[v] = r.x;
-        wp[v + 1] = r.y;
-      }
-      {
-        constexpr int v = 4;  // the fifth variable: its two sides as the pair
-        const float2 r = weno5x2(make_float2(u[v][0], u[v][4]), make_float2(u[v][1], u[v][3]),
-                                 make_float2(u[v][2], u[v][2]), make_float2(u[v][3], u[v][1]),
-                                 make_float2(u[v][4], u[v][0]), 1);
-        wm[v] = r.x;
-        wp[v] = r.y;
-      }
-    } else {
-#pragma unroll
-      for (int v = 0; v < 5; v += 2) {
-        const int w = v + 1 < 5 ? v + 1 : v;
-        const float2 r = weno5x2(make_float2(u[v][0], u[w][0]), make_float2(u[v][1], u[w][1]),
-                                 make_float2(u[v][2], u[w][2]), make_float2(u[v][3], u[w][3]),
-                                 make_float2(u[v][4], u[w][4]), textbook);
-        wm[v] = r.x;
-        if (v + 1 < 5) wm[v + 1] = r.y;
-      }
+    for (int v = 0; v < 4; v += 2) {
+      float2 l, r;
+      weno5x2_both(make_float2(u[v][0], u[v + 1][0]), make_float2(u[v][1], u[v + 1][1]),
+                   make_float2(u[v][2], u[v + 1][2]), make_float2(u[v][3], u[v + 1][3]),
+                   make_float2(u[v][4], u[v + 1][4]), l, r);
+      wm[v] = l.x;
+      wm[v + 1] = l.y;
+      wp[v] = r.x;
+      wp[v + 1] = r.y;
+    }
+    {
+      constexpr int v = 4;  // the fifth variable: its two sides as the pair
+      const float2 r = weno5x2(make_float2(u[v][0], u[v][4]), make_float2(u[v][1], u[v][3]),
+                               make_float2(u[v][2], u[v][2]), make_float2(u[v][3], u[v][1]),
+                               make_float2(u[v][4], u[v][0]), 1);
+      wm[v] = r.x;
+      wp[v] = r.y;
     }
   } else {
 #pragma unroll
     for (int v = 0; v < 5; ++v) {
       if constexpr (EX) {
-        wm[v] = weno5<R, EX, TB>(u[v][0], u[v][1], u[v][2], u[v][3], u[v][4], textbook);
-        if (TB) wp[v] = weno5<R, EX, TB>(u[v][4], u[v][3], u[v][2], u[v][1], u[v][0], 1);
+        wm[v] = weno5_exact<R>(u[v][0], u[v][1], u[v][2], u[v][3], u[v][4], textbook);
+        if (TB) wp[v] = weno5_exact<R>(u[v][4], u[v][3], u[v][2], u[v][1], u[v][0], 1);
       } else {
         const WenoParts w = weno5_parts<TB>(u[v][0], u[v][1], u[v][2], u[v][3], u[v][4]);
         wm[v] = weno5_left(w, u[v][2]);
