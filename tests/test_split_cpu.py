@@ -60,3 +60,51 @@ def test_even_split_covers_and_fits_in_few_tries(lib, blocks, slots, ovh):
     # cuts at most one column (another ovh): the mean and 4 plane-times more
     # always fits, 16 steps of a quarter from the first share tried.
     assert tries <= 17
+
+
+def split(lib, nz, slots, prec, ovh):
+    out = np.zeros((2 * len(nz) + 16 * slots, 3), np.int32)
+    n = lib.split_columns_c(len(nz), nz.ctypes.data_as(ctypes.c_void_p), slots, prec, ctypes.c_double(ovh),
+                            out.ctypes.data_as(ctypes.c_void_p), len(out))
+    assert n <= len(out)
+    return out[:n]
+
+
+# The branches of the split, each with a block that takes it on 148 SMs: the
+# precision form (0 exact, 1 FP64, 2 FP32), its tile, the resident CTAs of its
+# kernels per SM, and what is expected. The GPU tests run the same blocks.
+QUEUE, SPAN, ROUNDS, CHUNKS = "more tasks than CTAs", "shares over several columns", "two rounds", "equal chunks"
+BRANCHES = [
+    ((520, 300, 3), 1, (16, 8), 3, {QUEUE, SPAN}),
+    ((520, 300, 3), 0, (32, 8), 2, {QUEUE, SPAN}),
+    ((520, 300, 3), 2, (16, 8), 4, {QUEUE, SPAN}),
+    ((520, 300, 3), 2, (32, 8), 2, {QUEUE, SPAN}),
+    ((110, 110, 110), 2, (16, 8), 4, {CHUNKS}),
+    ((110, 110, 110), 2, (32, 8), 2, {CHUNKS}),
+    ((160, 152, 160), 1, (16, 8), 3, {QUEUE, ROUNDS}),
+    ((96, 104, 128), 0, (32, 8), 2, {QUEUE, ROUNDS}),
+    ((64, 48, 40), 1, (16, 8), 3, set()),
+]
+
+
+@pytest.mark.parametrize("ovh", [WENO, MUSCL])
+@pytest.mark.parametrize("n,prec,tile,per_sm,expected", BRANCHES)
+def test_every_branch_is_taken(lib, n, prec, tile, per_sm, expected, ovh):
+    nz, slots = columns(n, tx=tile[0], ty=tile[1]), 148 * per_sm
+    tasks = split(lib, nz, slots, prec, ovh)
+    check_cover(tasks, nz)
+    once, share, _ = even_split(lib, nz, slots, ovh)
+    twice, _, _ = even_split(lib, nz, 2 * slots, ovh)
+    got = set()
+    if len(tasks) > slots:
+        got.add(QUEUE)
+    if share > n[2] + ovh:
+        got.add(SPAN)
+    if np.array_equal(tasks, twice) and not np.array_equal(once, twice):
+        got.add(ROUNDS)
+    if np.ptp(tasks[:, 2] - tasks[:, 1]) <= 1 and not np.array_equal(tasks, once):
+        got.add(CHUNKS)
+        assert len(tasks) <= slots
+    if not got & {ROUNDS, CHUNKS}:
+        assert np.array_equal(tasks, once)
+    assert got == expected
