@@ -162,7 +162,7 @@ __global__ void finalize_kernel(const DevBlock* blocks, const DevCase* cases, co
 // ---------------------------------------------------------------- launchers
 static inline int grid_for(int64_t n, int bs) {
   int64_t g = (n + bs - 1) / bs;
-  if (g > 148 * 16) g = 148 * 16;
+  if (g > kNumSms * 16) g = kNumSms * 16;
   if (g < 1) g = 1;
   return (int)g;
 }
@@ -199,7 +199,7 @@ cudaError_t launch_init_dt(const DevBlock* blocks, int nblocks, int64_t max_cell
     // block, never fewer than 64 CTAs a block. With 64 for any block the first
     // step after an upload took 410 us more than the next on one block of
     // 160^3 cells and 256 us more on one of 128^3, now 134 and 97.
-    const int64_t most = std::max<int64_t>(64, std::min<int64_t>(148 * 8, 148 * 64 / nblocks));
+    const int64_t most = std::max<int64_t>(64, std::min<int64_t>(kNumSms * 8, kNumSms * 64 / nblocks));
     const int64_t gx = std::min<int64_t>(std::max<int64_t>(max_cells / 1024, 64), most);
     dim3 g((unsigned)gx, nblocks);
     wavespeed_kernel<<<g, 256, 0, s>>>(blocks, cases, role, case_max);

@@ -123,7 +123,7 @@ class Engine {
   std::string err;
   cudaStream_t stream = nullptr;
   int device = 0;
-  int num_sms = 148;
+  int num_sms = kNumSms;
   // resident CTAs per SM of each stage kernel at its shared-memory size,
   // found once (the attribute and the occupancy query cost a driver call
   // each, on every re-plan otherwise)

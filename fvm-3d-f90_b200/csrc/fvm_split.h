@@ -100,11 +100,17 @@ inline void split_columns(const std::vector<ZColumn>& cols, int slots, int prec,
   const size_t first = out.size();
   double share = even_split(cols, slots, ovh, out).share;
   // One round of shares is best (two: vortex 128^3 FP64 841 -> 870 us, 61x83x47
-  // blast 131 -> 142, 160^3 FP32 1009 -> 1035) until the FP64 forms' shares
-  // are so long that the CTAs drift apart by more than a second piece's
-  // warm-up costs: 64 planes (160^3 published form 1983 -> 1941), 16 in the
-  // exact form, whose planes take three times as long (vortex 100^3 2041 ->
-  // 1897).
+  // blast 131 -> 142, 64x64x256 404 -> 439, 160^3 FP32 1009 -> 1035, vortex 64^3
+  // exact 440 -> 495) until the FP64 forms' shares are so long that the CTAs
+  // drift apart by more than a second piece's warm-up costs: 64 planes
+  // (published form 160^3 2009 -> 1964, 192^3 3442 -> 3229, 256^3 5632 -> 5408;
+  // reference form 192^3 2729 -> 2631), 16 in the exact form, whose planes take
+  // three times as long (vortex 100^3 2039 -> 1897, 128^3 2734 -> 2693). Three
+  // rounds: 256^3 5320, but 192^3 3349 and 128^3 exact 2846. Where the columns
+  // outnumber the CTAs a share spans several of them and the second split only
+  // adds cuts: no difference beyond 1 % either way (64 blocks of 32 to 95 cells
+  // a side, FP64, 3867 -> 3863; exact, 24 to 64, 8703 -> 8606; 256^3 reference
+  // form 4252 -> 4280).
   if (prec != 2 && share >= (prec == 0 ? 16.0 : 64.0)) {
     out.resize(first);
     share = even_split(cols, 2 * slots, ovh, out).share;

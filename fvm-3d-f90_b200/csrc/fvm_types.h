@@ -19,6 +19,7 @@ namespace fvm {
 enum Role { ROLE_A = 0, ROLE_B = 1, ROLE_C = 2, ROLE_ACC = 3, NROLE = 4 };
 
 constexpr int kPadX = 4;   // left x pad (cells)
+constexpr int kNumSms = 148;  // SMs of a B200
 constexpr int kGhost = 3;  // ghost layers (defs_ghost_cell.f90:42, nGhost_layers = 3)
 
 // ghost_mask bit r (r = region-1, regions of defs_ghost_cell.f90:129-165):
@@ -98,12 +99,20 @@ struct StageArgs {
 // Programmatic dependent launch. Inside the step graphs the kernels of a time
 // step are launched with programmatic stream serialization, so the CTAs of a
 // launch are scheduled while the one before it drains. Every kernel of that
-// chain calls pdl_wait() before it touches global memory: it returns once the
-// preceding kernel has completed and its writes are visible (at once for a
-// kernel launched without the attribute). As every kernel of the chain waits,
-// the completion of one implies that of all before it. pdl_trigger() lets the
-// next launch be scheduled once every CTA of this one has started; it orders
-// no memory. Only the short gather and finalize kernels and one-round 2D stage
+// chain calls pdl_wait() before it touches anything that a kernel of the same
+// step writes: it returns once the preceding kernel has completed and its
+// writes are visible (at once for a kernel launched without the attribute). As
+// every kernel of the chain waits, the completion of one implies that of all
+// before it. Before the wait a kernel may read only
+//  * descriptors (tasks, blocks, cases, block lists), which copies of a re-plan
+//    write between steps: the stage and finalize kernels do;
+//  * the finalize alone, the case state of the step before: the previous
+//    finalize wrote it, and every stage kernel between the two has waited.
+// Both rest on one rule: no kernel calls pdl_trigger() before its own
+// pdl_wait(). Otherwise a launch could start two kernels early, before that
+// finalize has completed. pdl_trigger() lets the next launch be scheduled once
+// every CTA of this one has called it or exited; it orders no memory. Only the
+// short gather and finalize kernels and one-round 2D stage
 // launches trigger early, after their own wait: a launch scheduled behind a
 // long kernel's tail places its CTAs on the few SMs free at that moment (up to
 // 8 gather CTAs per SM) and runs unbalanced.

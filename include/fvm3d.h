@@ -239,8 +239,10 @@ int fvm_case_state(fvm_ctx* ctx, int case_id, double* t, double* dt, int64_t* st
 
 /* Autotuner hooks; no counterpart in the reference. fvm_tune_set forces the
  * tile shape (index 0: 32x8, 1: 16x16, 2: 32x8 with registers capped for two
- * resident CTAs per SM, 3: 16x8 on 128 threads, the heuristic's choice for 3D
- * FP32-flux and FP64 cases; -1 = heuristic) and z chunk length
+ * resident CTAs per SM, 3: 16x8 on 128 threads; -1 = heuristic: 2 for 2D and
+ * exact cases whose blocks are at least 32 wide and for FP32 WENO5 + AUSM in
+ * the reference's form where its padding costs less than 6 %, 1 for other
+ * exact cases, else 3) and z chunk length
  * (0 = heuristic) of the fused stage kernel for case `case_id`, keeping the
  * current state; fvm_tune_time_step runs `reps` full time steps (the state
  * advances) and returns the mean device time per step in ms.
