@@ -30,7 +30,7 @@ def evolve(mass_exp, prec, steps=3, **cfg):
 
 
 # At 2^-530 the product of density and pressure is below the normal range, at
-# 2^520 it overflows. The flux then takes another formula: a few hundred
+# 2^520 it overflows. Whatever formula the flux takes there, a few hundred
 # operations of half an ulp per step and component, three stages and three
 # steps, stay below 5000 half ulps, 6e-13, of the largest component.
 @pytest.mark.parametrize("exp", [-530, 520])
